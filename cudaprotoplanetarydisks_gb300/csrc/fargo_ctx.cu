@@ -160,6 +160,11 @@ KArgs<T> make_args(const fargo_ctx *c) {
   d.radmomm = (T *)c->radmomm;
   d.thetamomp = (T *)c->thetamomp;
   d.thetamomm = (T *)c->thetamomm;
+  // FP32's register azimuthal kernel takes the whole ring in before it writes: it
+  // works in place (two sets of momenta cost the 1024 x 3072 disk 1.4% in L2 misses)
+  void *apart[4] = {c->taurr, c->taurp, c->taupp, c->vthetaint};
+  void *in_place[4] = {c->radmomp, c->radmomm, c->thetamomp, c->thetamomm};
+  for (int k = 0; k < 4; k++) d.momr[k] = (T *)(sizeof(T) == 8 ? apart[k] : in_place[k]);
   d.sg_accr = (T *)c->sg_accr;
   d.sg_acct = (T *)c->sg_acct;
   d.az_scratch = (T *)c->az_scratch;
@@ -199,6 +204,7 @@ KArgs<T> make_args(const fargo_ctx *c) {
   a.mode = c->P.sloppy_cfl ? 2 : 0;
   a.az_smem = 0;
   a.az_regs = c->az_regs;
+  a.az_generic = c->az_generic ? 1 : 0;
   a.pdl = c->use_pdl ? 1 : 0;
   a.sg_generic = c->sg_generic ? 1 : 0;
   a.rad_maps = c->use_tma ? &c->rad_maps : nullptr;
@@ -450,12 +456,15 @@ int init_typed(fargo_ctx *c, const fargo_planet *planets) {
     size_t need = (size_t)AZ_NARR_HOST * p.nsec * E, need4 = (size_t)13 * p.nsec * E;
     const char *fg = std::getenv("FARGO_AZ_GLOBAL");  // force the global-memory ring buffers
     const bool force_global = fg && fg[0] == '1';
-    const bool force_generic = force_global || c->az_generic;  // the barrier-per-phase kernel
-    // register-blocked kernel when its ring fits in shared memory (chunks of four
-    // cells over at most 768 FP32 / 512 FP64 threads)
-    if (!force_generic && p.nsec % 4 == 0 && need4 + 1024 <= (size_t)maxsm) {
+    c->az_generic = c->az_generic || force_global;  // the barrier-per-phase kernel
+    // az_regs: the register-blocked FP32 kernel, when its ring fits in shared memory
+    // (chunks of four cells over at most 768 threads).  FP64 takes the warp kernel on
+    // every ring; its az_regs only says which rings the fused form carries
+    if (!c->az_generic && p.nsec % 4 == 0 && need4 + 1024 <= (size_t)maxsm) c->az_regs = 1;
+    if (!c->az_generic && E == 8) {
+      CK(prepare_kernels<T>(0, 0));
+    } else if (c->az_regs) {
       c->az_smem = need4;
-      c->az_regs = 1;
       CK(prepare_kernels<T>(need4, 1));
     } else if (!force_global && need + 1024 <= (size_t)maxsm) {
       c->az_smem = need;
@@ -1362,8 +1371,11 @@ int fused_build(fargo_fused *f, fargo_ctx *const *disks, int n, int by_width, st
   auto not_v4 = [&](const fargo_params &p, const fargo_ctx *c) { return !v4(p, c); };
   auto adiabatic = [](const fargo_params &p, const fargo_ctx *) { return p.adiabatic != 0; };
   auto corot = [](const fargo_params &p, const fargo_ctx *) { return p.corotating != 0; };
-  auto az_mc = [](const fargo_params &p, const fargo_ctx *) { return p.nsec / 4 > az4_threads_host<T>(p.nsec); };
+  auto az_mc = [](const fargo_params &p, const fargo_ctx *) { return sizeof(T) == 4 && p.nsec / 4 > az4_threads_host<T>(p.nsec); };
   auto az_one = [&](const fargo_params &p, const fargo_ctx *c) { return !az_mc(p, c); };
+  auto az_grid = [](const fargo_params &p, const fargo_ctx *) {
+    return make_int2(p.nrad, sizeof(T) == 8 ? azw_blocks_host(p.nsec) : 1);
+  };
   const dim3 b2(64, 4);
   std::vector<FusedGroup> head = {group(BK_DT_BEGIN, 0, all, one, dim3(32), 0, 0),
                                   group(BK_SOUNDSPEED, 0, adiabatic, rings, dim3(256), 0, 0)};
@@ -1376,7 +1388,7 @@ int fused_build(fargo_fused *f, fargo_ctx *const *disks, int n, int by_width, st
       const fargo_params &p = disks[k]->P;
       if (w && p.nsec != w) continue;
       if (v4(p, disks[k])) v4_threads = std::max(v4_threads, (p.nsec / 4 + 31) / 32 * 32);
-      az_threads = std::max(az_threads, az4_threads_host<T>(p.nsec));
+      az_threads = std::max(az_threads, sizeof(T) == 8 ? azw_threads_host(p.nsec) : az4_threads_host<T>(p.nsec));
       az_smem = std::max(az_smem, disks[k]->az_smem);
     }
     body.push_back({group(BK_CFL_V4, w, v4, rings, dim3(v4_threads), 0, 0),
@@ -1390,8 +1402,8 @@ int fused_build(fargo_fused *f, fargo_ctx *const *disks, int n, int by_width, st
                     group(BK_ENERGY, w, adiabatic, cells, b2, 0, 0, FUSED_CELL_MERGE),
                     group(BK_RADIAL, w, rad_tile, tiles, dim3(32, RAD_NY_HOST), rad_smem_bytes(sizeof(T)), 0),
                     group(BK_RADIAL_COL, w, rad_col, columns, dim3(RADC_THREADS), 0, 0),
-                    group(BK_AZ4, w, az_one, rings, dim3(az_threads), az_smem, 0),
-                    group(BK_AZ4_MC, w, az_mc, rings, dim3(sizeof(T) == 8 ? 512 : 768), az_smem, 0),
+                    group(BK_AZ4, w, az_one, az_grid, dim3(az_threads), az_smem, 0),
+                    group(BK_AZ4_MC, w, az_mc, rings, dim3(768), az_smem, 0),
                     group(BK_VELOCITIES, w, all, cells, b2, 0, 1, FUSED_CELL_MERGE),
                     group(BK_END, w, all, one, dim3(256), 0, 0)});
   }

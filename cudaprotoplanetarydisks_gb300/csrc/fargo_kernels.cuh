@@ -142,6 +142,9 @@ template <class T>
 cudaError_t prepare_batched(size_t rad_smem, size_t az_smem);
 template <class T>
 int az4_threads_host(int nsec);
+// the warp azimuthal kernel's blocks per ring and threads per block
+int azw_blocks_host(int nsec);
+int azw_threads_host(int nsec);
 #define RAD_NY_HOST 10
 size_t rad_smem_bytes(int esize);
 // CTAs of the persistent TMA radial transport on this device (0: not launchable)
