@@ -81,6 +81,7 @@ struct fargo_ctx {
   bool want_tma = true;       // the variant asks for the TMA radial transport
   int cell_block = 0;         // per-cell kernels' CTA shape (fargo_variant.cell_block)
   int az_chunks = 1;          // chunks per thread of the register azimuthal sweep
+  int rad_rings = 4;          // FP64: rings per chunk of the radial march
   bool rad_col = false;       // column-march radial transport
 };
 
@@ -105,18 +106,20 @@ void make_rad_maps(fargo_ctx *c) {
     return;
   const cuuint64_t dims[2] = {(cuuint64_t)c->P.nsec, (cuuint64_t)c->P.nrad + 1};
   const cuuint64_t strides[1] = {(cuuint64_t)c->P.nsec * E};
-  const cuuint32_t box[2] = {(cuuint32_t)RAD_BW(T), (cuuint32_t)RAD_BR};
+  // FP64: the march's stages (Vrad with the ring above them)
+  const cuuint32_t box[2] = {(cuuint32_t)(E == 4 ? RAD_BW : RADM_BW), (cuuint32_t)(E == 4 ? RAD_BR : RADM_STAGE)};
+  const cuuint32_t box_vr[2] = {box[0], box[1] + (E == 4 ? 0 : 1)};
   const cuuint32_t es[2] = {1, 1};
   const CUtensorMapDataType dt = E == 4 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_FLOAT64;
   void *src[4] = {c->dens, c->vrad, c->vtheta, c->P.adiabatic ? c->energy : c->dens};
   CUtensorMap *dst[4] = {&c->rad_maps.dens, &c->rad_maps.vrad, &c->rad_maps.vtheta, &c->rad_maps.energy};
   for (int f = 0; f < 4; f++) {
     if (!src[f]) return;
-    if (enc(dst[f], dt, 2, src[f], dims, strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
+    if (enc(dst[f], dt, 2, src[f], dims, strides, f == 1 ? box_vr : box, es, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
             CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
       return;
   }
-  c->rad_grid = rad_tma_grid<T>(c->P.nrad, c->P.nsec);
+  c->rad_grid = E == 4 ? rad_tma_grid(c->P.nrad, c->P.nsec) : 1;
   c->use_tma = c->rad_grid > 0;
 }
 
@@ -216,6 +219,7 @@ KArgs<T> make_args(const fargo_ctx *c) {
   }
   a.az_chunks = c->az_chunks;
   a.rad_col = c->rad_col ? 1 : 0;
+  a.rad_rings = c->rad_rings;
   a.cond_handle = 0;
   a.use_cond = 0;
   a.sg.spec_r = c->spec_r;
@@ -474,6 +478,12 @@ int init_typed(fargo_ctx *c, const fargo_planet *planets) {
       CK(prepare_kernels<T>(0, 0));
       if ((rc = dev_alloc(c, &c->az_scratch, (size_t)p.nrad * AZ_NARR_HOST * p.nsec * E))) return rc;
     }
+  }
+  {
+    int dev = 0, sms = 0;
+    CK(cudaGetDevice(&dev));
+    CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    c->rad_rings = radm_rings(p.nrad, p.nsec, sms);
   }
   // TMA maps of the radial transport's input fields
   if (c->want_tma) make_rad_maps<T>(c);
@@ -1359,14 +1369,15 @@ int fused_build(fargo_fused *f, fargo_ctx *const *disks, int n, int by_width, st
   auto one = [](const fargo_params &, const fargo_ctx *) { return make_int2(1, 1); };
   auto rings = [](const fargo_params &p, const fargo_ctx *) { return make_int2(p.nrad, 1); };
   auto cells = [](const fargo_params &p, const fargo_ctx *) { return make_int2((p.nsec + 63) / 64, (p.nrad + 3) / 4); };
-  auto tiles = [](const fargo_params &p, const fargo_ctx *) {
+  auto tiles = [](const fargo_params &p, const fargo_ctx *c) {
+    if (sizeof(T) == 8) return make_int2(radm_columns_host(p.nsec), (p.nrad + c->rad_rings - 1) / c->rad_rings);
     return make_int2((p.nsec + 31) / 32, (p.nrad + RAD_TR - 1) / RAD_TR);
   };
   auto columns = [](const fargo_params &p, const fargo_ctx *) {
     return make_int2((p.nsec + RADC_THREADS - 1) / RADC_THREADS, (p.nrad + RADC_RINGS - 1) / RADC_RINGS);
   };
-  auto rad_col = [](const fargo_params &, const fargo_ctx *c) { return c->rad_col; };
-  auto rad_tile = [](const fargo_params &, const fargo_ctx *c) { return !c->rad_col; };
+  auto rad_col = [](const fargo_params &, const fargo_ctx *c) { return sizeof(T) == 4 && c->rad_col; };
+  auto rad_tile = [](const fargo_params &, const fargo_ctx *c) { return sizeof(T) == 8 || !c->rad_col; };
   auto v4 = [](const fargo_params &p, const fargo_ctx *) { return p.nsec % 4 == 0 && p.nsec >= 260 && p.nsec <= 1024; };
   auto not_v4 = [&](const fargo_params &p, const fargo_ctx *c) { return !v4(p, c); };
   auto adiabatic = [](const fargo_params &p, const fargo_ctx *) { return p.adiabatic != 0; };
@@ -1400,14 +1411,15 @@ int fused_build(fargo_fused *f, fargo_ctx *const *disks, int n, int by_width, st
                     group(BK_VISC_UPDATE, w, all, cells, b2, 0, 0, FUSED_CELL_MERGE),
                     group(BK_ARTVISC, w, all, cells, b2, 0, 0, FUSED_CELL_MERGE),
                     group(BK_ENERGY, w, adiabatic, cells, b2, 0, 0, FUSED_CELL_MERGE),
-                    group(BK_RADIAL, w, rad_tile, tiles, dim3(32, RAD_NY_HOST), rad_smem_bytes(sizeof(T)), 0),
+                    group(BK_RADIAL, w, rad_tile, tiles, sizeof(T) == 8 ? dim3(RADM_THREADS) : dim3(32, RAD_NY_HOST),
+                          sizeof(T) == 8 ? 0 : rad_smem_bytes(), 0),
                     group(BK_RADIAL_COL, w, rad_col, columns, dim3(RADC_THREADS), 0, 0),
                     group(BK_AZ4, w, az_one, az_grid, dim3(az_threads), az_smem, 0),
                     group(BK_AZ4_MC, w, az_mc, rings, dim3(768), az_smem, 0),
                     group(BK_VELOCITIES, w, all, cells, b2, 0, 1, FUSED_CELL_MERGE),
                     group(BK_END, w, all, one, dim3(256), 0, 0)});
   }
-  if (prepare_batched<T>(rad_smem_bytes(sizeof(T)), az_smem_all) != cudaSuccess) {
+  if (prepare_batched<T>(rad_smem_bytes(), az_smem_all) != cudaSuccess) {
     *why = "cudaFuncSetAttribute on the batched kernels failed";
     return FARGO_ERR_CUDA;
   }

@@ -134,6 +134,15 @@ enum BatchKernel {
 // column-march radial transport: threads (sectors) per CTA, rings per thread
 #define RADC_THREADS 128
 #define RADC_RINGS 32
+// FP64 march: rings of a shared-memory stage, the box's sectors, the longest chunk, and
+// the work of a chunk's lead-in in rings
+#define RADM_THREADS 128
+#define RADM_STAGE 4
+#define RADM_BW 126
+#define RADM_MAX_RINGS 64
+#define RADM_LEAD 1.5
+int radm_rings(int nrad, int nsec, int sms);
+int radm_columns_host(int nsec);
 template <class T>
 void launch_batched(int kernel, const BatchGroup<T> &G, int nblocks, dim3 block, size_t smem, int pdl,
                     cudaStream_t s);
@@ -146,14 +155,13 @@ int az4_threads_host(int nsec);
 int azw_blocks_host(int nsec);
 int azw_threads_host(int nsec);
 #define RAD_NY_HOST 10
-size_t rad_smem_bytes(int esize);
+size_t rad_smem_bytes();
 // CTAs of the persistent TMA radial transport on this device (0: not launchable)
-template <class T>
 int rad_tma_grid(int nrad, int nsec);
-// TMA box of the radial transport's staged tiles: sectors (33 rounded up to 16
+// TMA box of the FP32 radial transport's staged tiles: sectors (33 rounded up to 16
 // bytes) x rings (the tile's RAD_TR rings, two below, three above)
 #define RAD_TR 16
-#define RAD_BW(T) (sizeof(T) == 4 ? 36 : 34)
+#define RAD_BW 36
 #define RAD_BR (RAD_TR + 5)
 
 // self-gravity (fargo_sg.cu)
