@@ -30,7 +30,7 @@ LIB_SOURCES = ["params.cpp", "setup.cpp", "fargo_kernels.cu", "fargo_sg.cu", "fa
                "fargo_noalloc.cu", "fargo_batch.cu", "fargo_mlp.cu", "fargo_learned.cu",
                "fargo_force_diag.cu", "fargo_peak.cu", "fargo_tc.cu"]
 EXE_SOURCES = ["driver.cpp"]
-HEADERS = ["fargo_internal.h", "fargo_device.cuh", "fargo_kernels.cuh"]
+HEADERS = ["fargo_internal.h", "fargo_physics.h", "fargo_device.cuh", "fargo_kernels.cuh"]
 
 
 def _obj(src):

@@ -45,7 +45,7 @@ struct fargo_ctx {
   void *densr = nullptr, *energyr = nullptr, *radmomp = nullptr, *radmomm = nullptr;
   void *thetamomp = nullptr, *thetamomm = nullptr, *sg_accr = nullptr, *sg_acct = nullptr;
   void *az_scratch = nullptr, *rt = nullptr, *nu = nullptr, *cosP = nullptr, *sinP = nullptr;
-  void *rdsum = nullptr;
+  void *rdsum = nullptr, *dcosP = nullptr;
   void *cosFt = nullptr, *sinFt = nullptr;
   double *rt64 = nullptr, *csmean = nullptr, *cosF = nullptr, *sinF = nullptr;
   double *ring_force = nullptr, *lostbydisk = nullptr;
@@ -182,6 +182,8 @@ KArgs<T> make_args(const fargo_ctx *c) {
   d.cosFt = (const T *)c->cosFt;
   d.sinFt = (const T *)c->sinFt;
   d.sinP = (const T *)c->sinP;
+  d.dcosP = (const T *)c->dcosP;
+  d.dsinP = c->dcosP ? (const T *)c->dcosP + c->P.nsec : nullptr;
   d.ring_force = c->ring_force;
   d.lostbydisk = c->lostbydisk;
   d.ctl = c->d_ctl;
@@ -447,6 +449,7 @@ int init_typed(fargo_ctx *c, const fargo_planet *planets) {
   if ((rc = dev_alloc(c, (void **)&c->sinF, (size_t)p.nsec * 8))) return rc;
   if ((rc = dev_alloc(c, &c->cosP, (size_t)p.nsec * E))) return rc;
   if ((rc = dev_alloc(c, &c->sinP, (size_t)p.nsec * E))) return rc;
+  if (E == 8 && (rc = dev_alloc(c, &c->dcosP, 2 * (size_t)p.nsec * E))) return rc;
   if ((rc = dev_alloc(c, &c->cosFt, (size_t)p.nsec * E))) return rc;
   if ((rc = dev_alloc(c, &c->sinFt, (size_t)p.nsec * E))) return rc;
   if ((rc = dev_alloc(c, (void **)&c->ring_force, n1 * (FARGO_MAXPL + 1) * 2 * 8))) return rc;
@@ -586,6 +589,16 @@ int init_typed(fargo_ctx *c, const fargo_planet *planets) {
   CK(cudaMemcpy(c->sinF, h.sinF.data(), (size_t)p.nsec * 8, cudaMemcpyHostToDevice));
   if ((rc = upload(c, c->cosP, h.cosP.data(), p.nsec))) return rc;
   if ((rc = upload(c, c->sinP, h.sinP.data(), p.nsec))) return rc;
+  if (E == 8) {
+    std::vector<double> dc(2 * (size_t)p.nsec);
+    const double k = 1.0 / (2.0 * FARGO_PI / (double)p.nsec);
+    for (int j = 0; j < p.nsec; j++) {
+      const int jm = j ? j - 1 : p.nsec - 1;
+      dc[j] = (h.cosP[j] - h.cosP[jm]) * k;
+      dc[p.nsec + j] = (h.sinP[j] - h.sinP[jm]) * k;
+    }
+    if ((rc = upload(c, c->dcosP, dc.data(), dc.size()))) return rc;
+  }
   if ((rc = upload(c, c->cosFt, h.cosF.data(), p.nsec))) return rc;
   if ((rc = upload(c, c->sinFt, h.sinF.data(), p.nsec))) return rc;
   if ((rc = upload(c, c->vrad, h.Vrad.data(), sg))) return rc;
@@ -622,6 +635,7 @@ int substep_typed(fargo_ctx *c, int which, double dt) {
   c->pin_ctl->dt = dt;
   c->pin_ctl->dt_sub = dt;
   c->pin_ctl->sloppy_dt = dt;
+  c->pin_ctl->diag = 1;
   if ((rc = write_ctl(c))) return rc;
   unsigned mask = 0;
   switch (which) {

@@ -34,6 +34,21 @@ enum RingTab {
   RT_CAVFAC,       // cavity factor of FViscosity (t = t0)
   RT_AZSHIFT,      // nsec/(2 pi Rmed): the FARGO shift per unit (Vtheta mean x dt)
   RT_INVSIGMAMED,  // 1/SigmaMed (0 where SigmaMed is 0)
+  // products of the rows above, formed once so that the FP64 kernels do not
+  RT_CS2,          // squared isothermal sound speed
+  RT_GRADP_R,      // 2 invdiffRmed, times gamma - 1 with the energy equation
+  RT_GRADP_T,      // 2/DXTHETA, times gamma - 1 or the squared sound speed
+  RT_STAR_R,       // (1/Rmed(i-1) - 1/Rmed(i)) invdiffRmed: radial gradient of the star's potential
+  RT_DIV_P, RT_DIV_M,    // Rsup, Rinf invdiffRsup/Rmed
+  RT_DPHI,               // 1/(dphi Rmed)
+  RT_HALF_INVRMED,       // 1/(2 Rmed)
+  RT_SHEAR_T, RT_SHEAR_R,  // Rinf invdiffRmed/4, 1/(4 dphi Rinf)
+  RT_VTRP_P, RT_VTRP_M,  // (Rsup invdiffRsup + 1/2)/Rmed, (1/2 - Rinf invdiffRsup)/Rmed
+  RT_VRRR_P, RT_VRRR_M,  // Rmed(i), Rmed(i-1) invdiffRmed/Rinf
+  RT_VRRP, RT_VRPP,      // 1/(dphi Rinf), 1/(2 Rinf)
+  RT_AV_R, RT_AV_T,      // 2 CVNR^2 invdiffRmed, 2 CVNR^2/DXTHETA
+  RT_AVE_R, RT_AVE_T,    // CVNR^2 invdiffRsup, CVNR^2/DXTHETA
+  RT_COOL_S, RT_COOL_I,  // EnergyMed/CoolingTime - QplusMed, 1/CoolingTime (0: no cooling time)
   RT_COUNT
 };
 

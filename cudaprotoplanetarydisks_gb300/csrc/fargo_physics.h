@@ -67,13 +67,17 @@ struct Ctl {
   // dt of the last substep that advanced the disk (a padded substep runs with
   // dt = 0), and the number of padded substeps run
   double dt_sub;
+  double invdt;               // 1 / dt (0 for dt = 0)
   long long padded;
   // ring means of the non-reflecting boundary: sound speed of rings 0, 1, nrad-1,
   // nrad-2, then density and energy of rings 0 and nrad-1 after the shift
   double bc_mean[8];
   // planetary system (Types.cuh:2-12)
   int nb;
-  int pad1;
+  // 1: the running substep is the last that a reader of the fields can see (the DT's last,
+  // a padded one, one with an error): the fields that no later substep reads
+  // (pressure, temperature, Q+, divergence) are written
+  int diag;
   double x[FARGO_MAXPL], y[FARGO_MAXPL], vx[FARGO_MAXPL], vy[FARGO_MAXPL];
   double mass[FARGO_MAXPL], acc[FARGO_MAXPL];
   int feeldisk[FARGO_MAXPL], feelothers[FARGO_MAXPL];
@@ -102,6 +106,7 @@ FARGO_HD void fargo_ctl_mirror(Ctl &c) {
   c.f32[CTL_F_INDX] = (float)c.ind_x;
   c.f32[CTL_F_INDY] = (float)c.ind_y;
   c.f32[CTL_F_DOMEGA] = (float)c.domega;
+  c.invdt = c.dt != 0.0 ? 1.0 / c.dt : 0.0;
   c.f32[CTL_F_INVDT] = c.dt != 0.0 ? 1.0f / (float)c.dt : 0.0f;
   c.ring_max[0] = c.ring_max[1] = FARGO_RING_NO_LIMIT;
 }

@@ -379,6 +379,33 @@ void host_ring_table(const fargo_params &p, const HostState &h, const DevParams 
     T(RT_SGSQRT, i) = (i < p.nrad) ? sqrt(h.Rmed[i] / h.Rmed[0]) : 0.0;
     T(RT_SGRATIO, i) = (i < p.nrad) ? h.Rmed[i] / h.Rmed[0] : 0.0;
     T(RT_CSMEAN, i) = at(h.cs_mean, i);
+    if (i < p.nrad) {
+      const double idphi = 1.0 / (2.0 * M_PI / (double)NSEC), gm1 = p.adiabatic ? p.adiabaticindex - 1.0 : 1.0;
+      const double ri = h.Rinf[i], rs = h.Rsup[i], idr = h.invdiffRmed[i], ids = h.invdiffRsup[i], irm = h.invRmed[i];
+      const double iri = h.invRinf[i], idx = T(RT_INVDXTHETA, i), cs = T(RT_CS, i), ct = T(RT_COOLTIME, i);
+      T(RT_CS2, i) = cs * cs;
+      T(RT_GRADP_R, i) = 2.0 * gm1 * idr;
+      T(RT_GRADP_T, i) = 2.0 * (p.adiabatic ? gm1 : cs * cs) * idx;
+      T(RT_STAR_R, i) = i > 0 ? (h.invRmed[i - 1] - irm) * idr : 0.0;
+      T(RT_DIV_P, i) = rs * ids * irm;
+      T(RT_DIV_M, i) = ri * ids * irm;
+      T(RT_DPHI, i) = idphi * irm;
+      T(RT_HALF_INVRMED, i) = 0.5 * irm;
+      T(RT_SHEAR_T, i) = 0.25 * ri * idr;
+      T(RT_SHEAR_R, i) = 0.25 * idphi * iri;
+      T(RT_VTRP_P, i) = (rs * ids + 0.5) * irm;
+      T(RT_VTRP_M, i) = (0.5 - ri * ids) * irm;
+      T(RT_VRRR_P, i) = h.Rmed[i] * idr * iri;
+      T(RT_VRRR_M, i) = i > 0 ? h.Rmed[i - 1] * idr * iri : 0.0;
+      T(RT_VRRP, i) = idphi * iri;
+      T(RT_VRPP, i) = 0.5 * iri;
+      T(RT_AV_R, i) = 2.0 * FARGO_CVNR * FARGO_CVNR * idr;
+      T(RT_AV_T, i) = 2.0 * FARGO_CVNR * FARGO_CVNR * idx;
+      T(RT_AVE_R, i) = FARGO_CVNR * FARGO_CVNR * ids;
+      T(RT_AVE_T, i) = FARGO_CVNR * FARGO_CVNR * idx;
+      T(RT_COOL_S, i) = ct > 0.0 ? T(RT_ENERGYMED, i) / ct - T(RT_QPLUSMED, i) : 0.0;
+      T(RT_COOL_I, i) = ct > 0.0 ? 1.0 / ct : 0.0;
+    }
     if (p.self_gravity && i < p.nrad) {
       double divRmed = h.Rmed[i] / h.Rmed[0];
       double normaccr = dp.sgp_rstep * dp.sgp_tstep / ((double)(2 * p.nrad) * (double)NSEC);
