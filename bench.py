@@ -195,6 +195,7 @@ def kernel_bytes(name, params, esize):
     khat = 2 * M * 2 * params.nrad * 16      # both kernel spectra
     fields = {
         "k_cfl_forces": (3 + ad) + (1 if True else 0),
+        "k_gas": (4 + ad + 2 * sg) + (2 + ad),
         "k_source": (4 + ad + 2 * sg) + 3,
         "k_visc_tau": 3 + 4,
         "k_visc_update": 6 + 2,

@@ -39,14 +39,17 @@ int fargo_batch_create_variant(int n, const fargo_params *params, const fargo_pl
   *out = nullptr;
   fargo_batch *b = new fargo_batch();
   int off = 0;
+  long long cells = 0;
+  for (int k = 0; k < n; k++) cells += (long long)params[k].nrad * params[k].nsec;
   for (int k = 0; k < n; k++) {
     if (nplanets[k] < 0 || (nplanets[k] > 0 && !planets)) {
       fargo_batch_destroy(b);
       return FARGO_ERR_INVALID;
     }
     fargo_ctx *c = nullptr;
-    const int rc = fargo_ctx_create_variant(&params[k], nplanets[k] ? planets + off : nullptr, nplanets[k],
-                                            precision, nullptr, v, &c);
+    const long long others = cells - (long long)params[k].nrad * params[k].nsec;
+    const int rc = fargo_ctx_create_among(&params[k], nplanets[k] ? planets + off : nullptr, nplanets[k], precision,
+                                          nullptr, v, others, &c);
     if (rc != FARGO_OK) {
       fargo_batch_destroy(b);
       return rc;

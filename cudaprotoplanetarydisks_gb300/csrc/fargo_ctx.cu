@@ -81,6 +81,9 @@ struct fargo_ctx {
   bool want_tma = true;       // the variant asks for the TMA radial transport
   int cell_block = 0;         // per-cell kernels' CTA shape (fargo_variant.cell_block)
   int az_chunks = 1;          // chunks per thread of the register azimuthal sweep
+  long long others = 0;       // cells of the disks that run at the same time (an ensemble)
+  bool gas = false;           // FP32, large grids: source step to energy equation by k_gas
+  int gas_rings = 4;          // its rings per chunk
   int rad_rings = 4;          // FP64: rings per chunk of the radial march
   bool rad_col = false;       // column-march radial transport
 };
@@ -88,40 +91,6 @@ struct fargo_ctx {
 namespace {
 // ring buffers of the barrier-per-phase azimuthal kernel (AZ_NARR in fargo_kernels.cu)
 constexpr int AZ_NARR_HOST = 12;
-
-// 2D tensor maps (sectors x rings 0..nrad, one box = RAD_BW sectors x RAD_BR rings,
-// zero fill outside) of the density, Vrad, Vtheta and (energy equation) energy,
-// for k_transport_radial_tma.  TMA needs 16-byte row strides (nsec * element size).
-// The encoder is the driver's cuTensorMapEncodeTiled, reached through the runtime.
-template <class T>
-void make_rad_maps(fargo_ctx *c) {
-  c->use_tma = false;
-  const size_t E = sizeof(T);
-  if (((size_t)c->P.nsec * E) % 16 != 0) return;
-  PFN_cuTensorMapEncodeTiled_v12000 enc = nullptr;
-  cudaDriverEntryPointQueryResult q;
-  if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", (void **)&enc, 12000, cudaEnableDefault, &q) !=
-          cudaSuccess ||
-      q != cudaDriverEntryPointSuccess || !enc)
-    return;
-  const cuuint64_t dims[2] = {(cuuint64_t)c->P.nsec, (cuuint64_t)c->P.nrad + 1};
-  const cuuint64_t strides[1] = {(cuuint64_t)c->P.nsec * E};
-  // FP64: the march's stages (Vrad with the ring above them)
-  const cuuint32_t box[2] = {(cuuint32_t)(E == 4 ? RAD_BW : RADM_BW), (cuuint32_t)(E == 4 ? RAD_BR : RADM_STAGE)};
-  const cuuint32_t box_vr[2] = {box[0], box[1] + (E == 4 ? 0 : 1)};
-  const cuuint32_t es[2] = {1, 1};
-  const CUtensorMapDataType dt = E == 4 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_FLOAT64;
-  void *src[4] = {c->dens, c->vrad, c->vtheta, c->P.adiabatic ? c->energy : c->dens};
-  CUtensorMap *dst[4] = {&c->rad_maps.dens, &c->rad_maps.vrad, &c->rad_maps.vtheta, &c->rad_maps.energy};
-  for (int f = 0; f < 4; f++) {
-    if (!src[f]) return;
-    if (enc(dst[f], dt, 2, src[f], dims, strides, f == 1 ? box_vr : box, es, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
-            CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
-      return;
-  }
-  c->rad_grid = E == 4 ? rad_tma_grid(c->P.nrad, c->P.nsec) : 1;
-  c->use_tma = c->rad_grid > 0;
-}
 
 int set_err(fargo_ctx *c, int code, const std::string &msg) {
   if (c) c->err = msg;
@@ -168,6 +137,14 @@ KArgs<T> make_args(const fargo_ctx *c) {
   void *apart[4] = {c->taurr, c->taurp, c->taupp, c->vthetaint};
   void *in_place[4] = {c->radmomp, c->radmomm, c->thetamomp, c->thetamomm};
   for (int k = 0; k < 4; k++) d.momr[k] = (T *)(sizeof(T) == 8 ? apart[k] : in_place[k]);
+  // k_gas leaves the new velocities in VradInt/VthetaInt and the new energy in a stress
+  // field, which it has no other use for; with boundary kernels in between, the energy
+  // equation runs after them and in place
+  const bool bc = c->P.open_inner || c->P.non_reflecting || c->P.evanescent;
+  d.energy_src = (T *)c->taurr;
+  d.tvr = (const T *)(c->gas ? c->vradint : c->vrad);
+  d.tvt = (const T *)(c->gas ? c->vthetaint : c->vtheta);
+  d.ten = (const T *)(c->gas && !bc && c->P.adiabatic ? c->taurr : c->energy);
   d.sg_accr = (T *)c->sg_accr;
   d.sg_acct = (T *)c->sg_acct;
   d.az_scratch = (T *)c->az_scratch;
@@ -222,6 +199,8 @@ KArgs<T> make_args(const fargo_ctx *c) {
   a.az_chunks = c->az_chunks;
   a.rad_col = c->rad_col ? 1 : 0;
   a.rad_rings = c->rad_rings;
+  a.gas = c->gas ? 1 : 0;
+  a.gas_rings = c->gas_rings;
   a.cond_handle = 0;
   a.use_cond = 0;
   a.sg.spec_r = c->spec_r;
@@ -246,6 +225,41 @@ KArgs<T> make_args(const fargo_ctx *c) {
   a.sg.nst0 = c->nst0;
   a.sg.M = c->P.nsec / 2 + 1;
   return a;
+}
+
+// 2D tensor maps (sectors x rings 0..nrad, one box = RAD_BW sectors x RAD_BR rings,
+// zero fill outside) of the density, Vrad, Vtheta and (energy equation) energy,
+// for k_transport_radial_tma.  TMA needs 16-byte row strides (nsec * element size).
+// The encoder is the driver's cuTensorMapEncodeTiled, reached through the runtime.
+template <class T>
+void make_rad_maps(fargo_ctx *c) {
+  c->use_tma = false;
+  const size_t E = sizeof(T);
+  if (((size_t)c->P.nsec * E) % 16 != 0) return;
+  PFN_cuTensorMapEncodeTiled_v12000 enc = nullptr;
+  cudaDriverEntryPointQueryResult q;
+  if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", (void **)&enc, 12000, cudaEnableDefault, &q) !=
+          cudaSuccess ||
+      q != cudaDriverEntryPointSuccess || !enc)
+    return;
+  const cuuint64_t dims[2] = {(cuuint64_t)c->P.nsec, (cuuint64_t)c->P.nrad + 1};
+  const cuuint64_t strides[1] = {(cuuint64_t)c->P.nsec * E};
+  // FP64: the march's stages (Vrad with the ring above them)
+  const cuuint32_t box[2] = {(cuuint32_t)(E == 4 ? RAD_BW : RADM_BW), (cuuint32_t)(E == 4 ? RAD_BR : RADM_STAGE)};
+  const cuuint32_t box_vr[2] = {box[0], box[1] + (E == 4 ? 0 : 1)};
+  const cuuint32_t es[2] = {1, 1};
+  const CUtensorMapDataType dt = E == 4 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_FLOAT64;
+  const KArgs<T> a = make_args<T>(c);
+  const void *src[4] = {a.d.dens, a.d.tvr, a.d.tvt, a.d.energy ? a.d.ten : a.d.dens};
+  CUtensorMap *dst[4] = {&c->rad_maps.dens, &c->rad_maps.vrad, &c->rad_maps.vtheta, &c->rad_maps.energy};
+  for (int f = 0; f < 4; f++) {
+    if (!src[f]) return;
+    if (enc(dst[f], dt, 2, const_cast<void *>(src[f]), dims, strides, f == 1 ? box_vr : box, es, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
+            CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
+      return;
+  }
+  c->rad_grid = E == 4 ? rad_tma_grid(c->P.nrad, c->P.nsec) : 1;
+  c->use_tma = c->rad_grid > 0;
 }
 
 int dev_alloc(fargo_ctx *c, void **p, size_t bytes) {
@@ -487,6 +501,13 @@ int init_typed(fargo_ctx *c, const fargo_planet *planets) {
     CK(cudaGetDevice(&dev));
     CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     c->rad_rings = radm_rings(p.nrad, p.nsec, sms);
+    // k_gas where the disks that run at the same time have a million cells: below, its
+    // blocks are too few to hide a march's latency (one disk of 512 x 1536: a substep 98 us
+    // with the cell kernels, 109 with k_gas; 640 x 1920: 58 against 49 ms for five DTs; 1024 x 3072: 380
+    // against 344 us; 32 disks of 128 to 512 rings: 207 against 172 ms for five DTs).  In an ensemble the
+    // disks fill the GPU together and chunks of 16 rings measured best (8 .. 64).
+    c->gas = E == 4 && (long long)p.nrad * p.nsec + c->others >= GAS_CELLS;
+    c->gas_rings = c->others ? 16 : gas_rings(p.nrad, p.nsec, sms);
   }
   // TMA maps of the radial transport's input fields
   if (c->want_tma) make_rad_maps<T>(c);
@@ -800,6 +821,11 @@ int fargo_ctx_create(const fargo_params *p, const fargo_planet *planets, int nb,
 
 int fargo_ctx_create_variant(const fargo_params *p, const fargo_planet *planets, int nb, int precision, void *stream,
                              const fargo_variant *variant, fargo_ctx **out) {
+  return fargo_ctx_create_among(p, planets, nb, precision, stream, variant, 0, out);
+}
+
+int fargo_ctx_create_among(const fargo_params *p, const fargo_planet *planets, int nb, int precision, void *stream,
+                           const fargo_variant *variant, long long others, fargo_ctx **out) {
   if (!p || !out || nb < 0 || nb > FARGO_MAXPL || (nb > 0 && !planets)) return FARGO_ERR_INVALID;
   fargo_variant v;
   if (variant) v = *variant;
@@ -814,6 +840,7 @@ int fargo_ctx_create_variant(const fargo_params *p, const fargo_planet *planets,
   c->nb = nb;
   c->precision = precision;
   c->esize = precision == FARGO_FP64 ? 8 : 4;
+  c->others = others;
   c->dp = host_dev_params(*p, nb);
   c->use_graph = v.graph != 0;
   c->use_pdl = v.pdl != 0;
@@ -1303,7 +1330,7 @@ constexpr int FUSED_CELL_MERGE = 4;
 const char *batch_kernel_name(int k) {
   static const char *const names[BK_END + 1] = {
       "kb_dt_begin", "kb_soundspeed", "kb_cfl_forces (4 cells/thread)", "kb_cfl_forces", "kb_planets",
-      "kb_correct_vtheta", "kb_source", "kb_visc_tau", "kb_visc_update", "kb_artvisc", "kb_energy", "kb_radial",
+      "kb_correct_vtheta", "kb_source", "kb_visc_tau", "kb_visc_update", "kb_artvisc", "kb_energy", "kb_gas", "kb_radial",
       "kb_radial_col", "kb_azimuthal4", "kb_azimuthal4 (chunks/thread)", "kb_velocities", "kb_end"};
   return k >= 0 && k <= BK_END ? names[k] : "?";
 }
@@ -1395,6 +1422,12 @@ int fused_build(fargo_fused *f, fargo_ctx *const *disks, int n, int by_width, st
   auto v4 = [](const fargo_params &p, const fargo_ctx *) { return p.nsec % 4 == 0 && p.nsec >= 260 && p.nsec <= 1024; };
   auto not_v4 = [&](const fargo_params &p, const fargo_ctx *c) { return !v4(p, c); };
   auto adiabatic = [](const fargo_params &p, const fargo_ctx *) { return p.adiabatic != 0; };
+  auto gas = [](const fargo_params &, const fargo_ctx *c) { return c->gas; };
+  auto parts = [](const fargo_params &, const fargo_ctx *c) { return !c->gas; };
+  auto parts_energy = [](const fargo_params &p, const fargo_ctx *c) { return !c->gas && p.adiabatic != 0; };
+  auto gas_grid = [](const fargo_params &p, const fargo_ctx *c) {
+    return make_int2(gas_columns_host(p.nsec), (p.nrad + c->gas_rings - 1) / c->gas_rings);
+  };
   auto corot = [](const fargo_params &p, const fargo_ctx *) { return p.corotating != 0; };
   auto az_mc = [](const fargo_params &p, const fargo_ctx *) { return sizeof(T) == 4 && p.nsec / 4 > az4_threads_host<T>(p.nsec); };
   auto az_one = [&](const fargo_params &p, const fargo_ctx *c) { return !az_mc(p, c); };
@@ -1420,11 +1453,12 @@ int fused_build(fargo_fused *f, fargo_ctx *const *disks, int n, int by_width, st
                     group(BK_CFL, w, not_v4, rings, dim3(256), 0, 0),
                     group(BK_PLANETS, w, all, one, dim3(64), 0, 0),
                     group(BK_COROT, w, corot, cells, b2, 0, 0, FUSED_CELL_MERGE),
-                    group(BK_SOURCE, w, all, cells, b2, 0, 0, FUSED_CELL_MERGE),
-                    group(BK_VISC_TAU, w, all, cells, b2, 0, 0, FUSED_CELL_MERGE),
-                    group(BK_VISC_UPDATE, w, all, cells, b2, 0, 0, FUSED_CELL_MERGE),
-                    group(BK_ARTVISC, w, all, cells, b2, 0, 0, FUSED_CELL_MERGE),
-                    group(BK_ENERGY, w, adiabatic, cells, b2, 0, 0, FUSED_CELL_MERGE),
+                    group(BK_SOURCE, w, parts, cells, b2, 0, 0, FUSED_CELL_MERGE),
+                    group(BK_VISC_TAU, w, parts, cells, b2, 0, 0, FUSED_CELL_MERGE),
+                    group(BK_VISC_UPDATE, w, parts, cells, b2, 0, 0, FUSED_CELL_MERGE),
+                    group(BK_ARTVISC, w, parts, cells, b2, 0, 0, FUSED_CELL_MERGE),
+                    group(BK_ENERGY, w, parts_energy, cells, b2, 0, 0, FUSED_CELL_MERGE),
+                    group(BK_GAS, w, gas, gas_grid, dim3(GAS_THREADS), 0, 0),
                     group(BK_RADIAL, w, rad_tile, tiles, sizeof(T) == 8 ? dim3(RADM_THREADS) : dim3(32, RAD_NY_HOST),
                           sizeof(T) == 8 ? 0 : rad_smem_bytes(), 0),
                     group(BK_RADIAL_COL, w, rad_col, columns, dim3(RADC_THREADS), 0, 0),

@@ -92,6 +92,9 @@ struct DiskView {
   double *ring;
   void *cand;
 };
+// fargo_ctx_create_variant for a disk that runs beside others of that many cells together
+extern "C" int fargo_ctx_create_among(const fargo_params *p, const fargo_planet *planets, int nb, int precision, void *stream,
+                                      const fargo_variant *variant, long long others, fargo_ctx **out);
 extern "C" int fargo_disk_view(fargo_ctx *c, DiskView *v);
 
 // output.cpp

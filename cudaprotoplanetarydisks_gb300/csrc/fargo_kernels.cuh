@@ -129,11 +129,17 @@ struct BatchGroup {
 };
 enum BatchKernel {
   BK_DT_BEGIN, BK_SOUNDSPEED, BK_CFL_V4, BK_CFL, BK_PLANETS, BK_COROT, BK_SOURCE, BK_VISC_TAU,
-  BK_VISC_UPDATE, BK_ARTVISC, BK_ENERGY, BK_RADIAL, BK_RADIAL_COL, BK_AZ4, BK_AZ4_MC, BK_VELOCITIES, BK_END
+  BK_VISC_UPDATE, BK_ARTVISC, BK_ENERGY, BK_GAS, BK_RADIAL, BK_RADIAL_COL, BK_AZ4, BK_AZ4_MC, BK_VELOCITIES, BK_END
 };
 // column-march radial transport: threads (sectors) per CTA, rings per thread
 #define RADC_THREADS 128
 #define RADC_RINGS 32
+// k_gas: threads (sectors and halo) per CTA, the longest chunk
+#define GAS_THREADS 128
+#define GAS_MAX_RINGS 64
+#define GAS_CELLS 1000000
+int gas_rings(int nrad, int nsec, int sms);
+int gas_columns_host(int nsec);
 // FP64 march: rings of a shared-memory stage, the box's sectors, the longest chunk, and
 // the work of a chunk's lead-in in rings
 #define RADM_THREADS 128
