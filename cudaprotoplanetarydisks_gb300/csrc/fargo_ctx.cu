@@ -45,7 +45,7 @@ struct fargo_ctx {
   void *densr = nullptr, *energyr = nullptr, *radmomp = nullptr, *radmomm = nullptr;
   void *thetamomp = nullptr, *thetamomm = nullptr, *sg_accr = nullptr, *sg_acct = nullptr;
   void *az_scratch = nullptr, *rt = nullptr, *nu = nullptr, *cosP = nullptr, *sinP = nullptr;
-  void *rdsum = nullptr, *dcosP = nullptr;
+  void *rdsum = nullptr, *dcosP = nullptr, *mom_extra[2] = {nullptr, nullptr};
   void *cosFt = nullptr, *sinFt = nullptr;
   double *rt64 = nullptr, *csmean = nullptr, *cosF = nullptr, *sinF = nullptr;
   double *ring_force = nullptr, *lostbydisk = nullptr;
@@ -57,6 +57,7 @@ struct fargo_ctx {
   int rad1[16], nst1 = 0, rad0[16], nst0 = 0;
   size_t az_smem = 0;
   int az_regs = 0;
+  bool az_warp32 = false;     // FP32 rings of nsec % 4 != 0: the warp azimuthal kernel
   double *staging = nullptr;   // FP64 staging slots of host <-> device transfers (FP32 fields)
   double *lx_rmed = nullptr, *lx_surf = nullptr, *lx_ring = nullptr;  // learned correction (first use)
   void *lx_cand = nullptr;
@@ -134,9 +135,10 @@ KArgs<T> make_args(const fargo_ctx *c) {
   d.thetamomm = (T *)c->thetamomm;
   // FP32's register azimuthal kernel takes the whole ring in before it writes: it
   // works in place (two sets of momenta cost the 1024 x 3072 disk 1.4% in L2 misses)
-  void *apart[4] = {c->taurr, c->taurp, c->taupp, c->vthetaint};
+  // (the warp kernels' blocks of one ring read what others write, and keep them apart)
+  void *apart[4] = {c->gas ? c->mom_extra[0] : c->taurr, c->taurp, c->taupp, c->gas ? c->mom_extra[1] : c->vthetaint};
   void *in_place[4] = {c->radmomp, c->radmomm, c->thetamomp, c->thetamomm};
-  for (int k = 0; k < 4; k++) d.momr[k] = (T *)(sizeof(T) == 8 ? apart[k] : in_place[k]);
+  for (int k = 0; k < 4; k++) d.momr[k] = (T *)(sizeof(T) == 8 || c->az_warp32 ? apart[k] : in_place[k]);
   // k_gas leaves the new velocities in VradInt/VthetaInt and the new energy in a stress
   // field, which it has no other use for; with boundary kernels in between, the energy
   // equation runs after them and in place
@@ -186,6 +188,7 @@ KArgs<T> make_args(const fargo_ctx *c) {
   a.mode = c->P.sloppy_cfl ? 2 : 0;
   a.az_smem = 0;
   a.az_regs = c->az_regs;
+  a.az_warp32 = c->az_warp32 ? 1 : 0;
   a.az_generic = c->az_generic ? 1 : 0;
   a.pdl = c->use_pdl ? 1 : 0;
   a.sg_generic = c->sg_generic ? 1 : 0;
@@ -482,7 +485,8 @@ int init_typed(fargo_ctx *c, const fargo_planet *planets) {
     // (chunks of four cells over at most 768 threads).  FP64 takes the warp kernel on
     // every ring; its az_regs only says which rings the fused form carries
     if (!c->az_generic && p.nsec % 4 == 0 && need4 + 1024 <= (size_t)maxsm) c->az_regs = 1;
-    if (!c->az_generic && E == 8) {
+    c->az_warp32 = !c->az_generic && E == 4 && p.nsec % 4 != 0;
+    if (!c->az_generic && (E == 8 || c->az_warp32)) {
       CK(prepare_kernels<T>(0, 0));
     } else if (c->az_regs) {
       c->az_smem = need4;
@@ -507,6 +511,8 @@ int init_typed(fargo_ctx *c, const fargo_planet *planets) {
     // against 344 us; 32 disks of 128 to 512 rings: 207 against 172 ms for five DTs).  In an ensemble the
     // disks fill the GPU together and chunks of 16 rings measured best (8 .. 64).
     c->gas = E == 4 && (long long)p.nrad * p.nsec + c->others >= GAS_CELLS;
+    for (int k = 0; k < 2 && c->gas && c->az_warp32; k++)
+      if ((rc = dev_alloc(c, &c->mom_extra[k], sg * E))) return rc;
     c->gas_rings = c->others ? 16 : gas_rings(p.nrad, p.nsec, sms);
   }
   // TMA maps of the radial transport's input fields
