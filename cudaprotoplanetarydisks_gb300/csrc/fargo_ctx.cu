@@ -360,6 +360,7 @@ int device_error(fargo_ctx *c) {
 template <class T>
 int build_graph(fargo_ctx *c) {
   KArgs<T> a = make_args<T>(c);
+  a.cs_ready = 1;  // the prefix forms it
   cudaGraph_t g = nullptr, gp = nullptr;
   CK(cudaGraphCreate(&g, 0));
   LaunchProbe probe;
@@ -414,6 +415,7 @@ int build_graph(fargo_ctx *c) {
 template <class T>
 int run_dt_hostloop(fargo_ctx *c) {
   KArgs<T> a = make_args<T>(c);
+  a.cs_ready = 1;  // the prefix forms it
   const bool ahead = c->use_sg_ahead && sg_ahead_allowed<T>(a, &c->side);
   launch_dt_prefix<T>(a, c->stream);
   if (ahead) launch_sg_rows_fwd<T>(a, c->stream);
@@ -735,6 +737,7 @@ int cfl_typed(fargo_ctx *c, double deltaT, int *cfl) {
 template <class T>
 int time_kernels_typed(fargo_ctx *c, int reps, std::vector<double> &ms) {
   KArgs<T> a = make_args<T>(c);
+  a.cs_ready = 1;  // the prefix forms it
   LaunchProbe probe;
   std::memset(&probe, 0, sizeof(probe));
   probe.nev = 96;

@@ -113,8 +113,9 @@ template <class T>
 void launch_dt_prefix(const KArgs<T> &a, cudaStream_t s);
 template <class T>
 void launch_cfl_only(const KArgs<T> &a, cudaStream_t s);
+// cs_known: the sound speed holds but for the rings that a non-reflecting boundary sets
 template <class T>
-void launch_boundaries(const KArgs<T> &a, cudaStream_t s);
+void launch_boundaries(const KArgs<T> &a, cudaStream_t s, bool cs_known = false);
 template <class T>
 cudaError_t prepare_kernels(size_t az_smem_bytes, int az_regs);
 // Fused ensembles: one launch of a substep kernel over a group of disks

@@ -69,9 +69,9 @@ struct Ctl {
   double dt_sub;
   double invdt;               // 1 / dt (0 for dt = 0)
   long long padded;
-  // ring means of the non-reflecting boundary: sound speed of rings 0, 1, nrad-1,
-  // nrad-2, then density and energy of rings 0 and nrad-1 after the shift
-  double bc_mean[8];
+  // ring means of the non-reflecting boundary: density of rings 1 and nrad-2, then
+  // energy
+  double bc_mean[4];
   // planetary system (Types.cuh:2-12)
   int nb;
   // 1: the running substep is the last that a reader of the fields can see (the DT's last,
