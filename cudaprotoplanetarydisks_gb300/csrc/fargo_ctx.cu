@@ -140,13 +140,12 @@ KArgs<T> make_args(const fargo_ctx *c) {
   void *in_place[4] = {c->radmomp, c->radmomm, c->thetamomp, c->thetamomm};
   for (int k = 0; k < 4; k++) d.momr[k] = (T *)(sizeof(T) == 8 || c->az_warp32 ? apart[k] : in_place[k]);
   // k_gas leaves the new velocities in VradInt/VthetaInt and the new energy in a stress
-  // field, which it has no other use for; with boundary kernels in between, the energy
-  // equation runs after them and in place
-  const bool bc = c->P.open_inner || c->P.non_reflecting || c->P.evanescent;
+  // field, which it has no other use for; the evanescent boundary sets rings all over the
+  // disk in between, and the energy equation runs after it and in place
   d.energy_src = (T *)c->taurr;
   d.tvr = (const T *)(c->gas ? c->vradint : c->vrad);
   d.tvt = (const T *)(c->gas ? c->vthetaint : c->vtheta);
-  d.ten = (const T *)(c->gas && !bc && c->P.adiabatic ? c->taurr : c->energy);
+  d.ten = (const T *)(c->gas && !c->P.evanescent && c->P.adiabatic ? c->taurr : c->energy);
   d.sg_accr = (T *)c->sg_accr;
   d.sg_acct = (T *)c->sg_acct;
   d.az_scratch = (T *)c->az_scratch;
