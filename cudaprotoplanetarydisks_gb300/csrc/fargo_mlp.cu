@@ -494,12 +494,12 @@ __global__ void __launch_bounds__(TCF_THREADS) k_mlp_forward_tc(const float *__r
 struct MlpBwdSmem {
   MlpFwdW f;
   MlpBwdW b;
-  bf16 xs[MLP_ROWS][MLP_LDX];    // X of the tile
+  bf16 xs2[2][MLP_ROWS][MLP_LDX];  // X of the tile, and of the next one while this is in work
   bf16 h1s[MLP_ROWS][MLP_LDH];   // GELU(z1)
   bf16 h2s[MLP_ROWS][MLP_LDH];   // GELU(z2)
   bf16 dz1s[MLP_ROWS][MLP_LDH];  // dL/dz1 (BF16)
   bf16 dz2s[MLP_ROWS][MLP_LDH];
-  bf16 dys[MLP_ROWS][8];         // dL/dy (BF16), columns 2..7 zero
+  bf16 dys2[2][MLP_ROWS][8];       // dL/dy (BF16), columns 2..7 zero
 };
 
 __global__ void __launch_bounds__(128, 2) k_mlp_backward(const float *__restrict__ P, const bf16 *__restrict__ X,
@@ -519,28 +519,38 @@ __global__ void __launch_bounds__(128, 2) k_mlp_backward(const float *__restrict
   float accb = 0.0f, accb3 = 0.0f;  // bias sums of the thread's column
   const int ntile = (n + MLP_ROWS - 1) / MLP_ROWS;
   const int rw = 16 * w;  // the warp's rows within the tile
-  for (int tile = blockIdx.x; tile < ntile; tile += gridDim.x) {
+  // a tile's X into buffer b (cp.async); its dy into a register, for the buffer when this tile is done
+  auto fetch = [&](int tile, int b) {
     const int R0 = tile * MLP_ROWS;
     for (int c = tid; c < MLP_ROWS * 16; c += blockDim.x) {
       const int row = c >> 4, col = (c & 15) * 8;
       const bool valid = R0 + row < n;
-      cp_async16(&s.xs[row][col], X + (size_t)(valid ? R0 + row : 0) * MLP_IN + col, valid);
+      cp_async16(&s.xs2[b][row][col], X + (size_t)(valid ? R0 + row : 0) * MLP_IN + col, valid);
     }
     cp_async_commit();
-    if (tid < MLP_ROWS) {
-      const bool valid = R0 + tid < n;
-      const float2 d =
-          valid ? *reinterpret_cast<const float2 *>(dy + (size_t)(R0 + tid) * MLP_OUT) : make_float2(0.0f, 0.0f);
-      *reinterpret_cast<uint4 *>(&s.dys[tid][0]) = make_uint4(pack2(d.x, d.y), 0u, 0u, 0u);
-    }
+    const bool valid = tid < MLP_ROWS && R0 + tid < n;
+    return valid ? *reinterpret_cast<const float2 *>(dy + (size_t)(R0 + tid) * MLP_OUT) : make_float2(0.0f, 0.0f);
+  };
+  auto put_dy = [&](float2 d, int b) {
+    if (tid < MLP_ROWS) *reinterpret_cast<uint4 *>(&s.dys2[b][tid][0]) = make_uint4(pack2(d.x, d.y), 0u, 0u, 0u);
+  };
+  int b = 0;
+  if ((int)blockIdx.x < ntile) put_dy(fetch(blockIdx.x, 0), 0);
+  for (int tile = blockIdx.x; tile < ntile; tile += gridDim.x, b ^= 1) {
+    bf16(*const xs)[MLP_LDX] = s.xs2[b];
+    bf16(*const dys)[8] = s.dys2[b];
     cp_async_wait<0>();
     __syncthreads();
+    // the next tile's rows stream in behind this one's work (their buffer was last read before the barrier)
+    const bool more = tile + (int)gridDim.x < ntile;
+    float2 next = make_float2(0.0f, 0.0f);
+    if (more) next = fetch(tile + gridDim.x, b ^ 1);
     // ---- data gradients of the warp's 16 rows
     {
       unsigned z1p[8][2], z2p[8][2], h2[4][4];
-      layers12<false>(s.f, &s.xs[rw][0], lane, z1p, z2p, h2, &s.h1s[rw][0], &s.h2s[rw][0]);
+      layers12<false>(s.f, &xs[rw][0], lane, z1p, z2p, h2, &s.h1s[rw][0], &s.h2s[rw][0]);
       // dh2 = dy W3^T: A = dy (16 x 16, columns >= 8 zero)
-      const unsigned a[4] = {ld_u32(&s.dys[rw + g][2 * t]), ld_u32(&s.dys[rw + g + 8][2 * t]), 0u, 0u};
+      const unsigned a[4] = {ld_u32(&dys[rw + g][2 * t]), ld_u32(&dys[rw + g + 8][2 * t]), 0u, 0u};
       float c[8][4];
 #pragma unroll
       for (int np = 0; np < 4; np++) {
@@ -597,7 +607,7 @@ __global__ void __launch_bounds__(128, 2) k_mlp_backward(const float *__restrict
 #pragma unroll
       for (int mi = 0; mi < 2; mi++) {
         unsigned a[4];
-        ldsm_x4_t(a, &s.xs[k0 + rr + 8 * (q >> 1)][(2 * w + mi) * 16 + 8 * (q & 1)]);
+        ldsm_x4_t(a, &xs[k0 + rr + 8 * (q >> 1)][(2 * w + mi) * 16 + 8 * (q & 1)]);
 #pragma unroll
         for (int np = 0; np < 4; np++) {
           mma16816(acc1[mi][2 * np], a, &b1[np][0]);
@@ -616,7 +626,7 @@ __global__ void __launch_bounds__(128, 2) k_mlp_backward(const float *__restrict
       }
       ldsm_x4_t(a, &s.h2s[k0 + rr + 8 * (q >> 1)][w * 16 + 8 * (q & 1)]);
       unsigned b3[2];
-      ldsm_x2_t(b3, &s.dys[k0 + rr + 8 * (q & 1)][0]);
+      ldsm_x2_t(b3, &dys[k0 + rr + 8 * (q & 1)][0]);
       mma16816(acc3, a, b3);
     }
     // bias gradients: column sums over the tile's rows, in row order
@@ -628,11 +638,12 @@ __global__ void __launch_bounds__(128, 2) k_mlp_backward(const float *__restrict
       accb += v;
       if (tid < MLP_OUT) {
         float u = 0.0f;
-        for (int r = 0; r < MLP_ROWS; r++) u += __bfloat162float(s.dys[r][tid]);
+        for (int r = 0; r < MLP_ROWS; r++) u += __bfloat162float(dys[r][tid]);
         accb3 += u;
       }
     }
-    __syncthreads();  // the tile buffers are refilled next
+    if (more) put_dy(next, b ^ 1);
+    __syncthreads();  // the tile's gradients are refilled next
   }
   float *out = part + (size_t)blockIdx.x * MLP_NPARAM;
 #pragma unroll
@@ -666,13 +677,35 @@ __global__ void __launch_bounds__(128, 2) k_mlp_backward(const float *__restrict
   if (tid < MLP_OUTP) out[MLP_OFF_B3 + tid] = tid < MLP_OUT ? accb3 : 0.0f;
 }
 
-// grad[p] = sum over CTAs c of part[c][p], in CTA order (deterministic)
-__global__ void k_mlp_reduce(const float *__restrict__ part, int nparts, float *__restrict__ grad) {
-  const int p = blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= MLP_NPARAM) return;
-  double acc = 0.0;
-  for (int c = 0; c < nparts; c++) acc += (double)part[(size_t)c * MLP_NPARAM + p];
-  grad[p] = (float)acc;
+// grad[p] = sum over CTAs c of part[c][p], in a fixed order (deterministic).  A block takes 32
+// parameters; its warp w sums the CTAs w, w + RED_WARPS, ... and the warps' sums are added
+// in order.  The sums are float pairs (Knuth's TwoSum, some 48 bits: rounded to FP32 the
+// FP64 sum's value): this GPU converts 0.6 floats to double per clock and SM, and with one thread
+// per parameter and FP64 sums the conversions and 304 dependent loads took 40 us, now 4 us.
+#define RED_WARPS 8
+struct Sum2 {
+  float hi, lo;
+  __device__ __forceinline__ void add(float x, float xl) {
+    const float t = hi + x, b = t - hi;
+    lo += ((hi - (t - b)) + (x - b)) + xl;
+    hi = t;
+  }
+};
+__global__ void __launch_bounds__(32 * RED_WARPS) k_mlp_reduce(const float *__restrict__ part, int nparts,
+                                                               float *__restrict__ grad) {
+  __shared__ Sum2 sh[RED_WARPS][32];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, p = blockIdx.x * 32 + lane;
+  Sum2 s = {0.0f, 0.0f};
+  if (p < MLP_NPARAM) {
+#pragma unroll 8
+    for (int c = w; c < nparts; c += RED_WARPS) s.add(part[(size_t)c * MLP_NPARAM + p], 0.0f);
+  }
+  sh[w][lane] = s;
+  __syncthreads();
+  if (w != 0 || p >= MLP_NPARAM) return;
+#pragma unroll
+  for (int k = 1; k < RED_WARPS; k++) s.add(sh[k][lane].hi, sh[k][lane].lo);
+  grad[p] = s.hi + s.lo;
 }
 
 // Adam (Kingma & Ba 2015) on the FP32 master weights; the padded columns of the
@@ -828,7 +861,7 @@ int fargo_mlp_backward(fargo_mlp *m, const void *x, int n, const float *dy, void
   const cudaStream_t s = (cudaStream_t)stream;
   const int ctas = std::min(m->bwd_ctas, (n + MLP_ROWS - 1) / MLP_ROWS);
   k_mlp_backward<<<ctas, 128, bwd_smem(), s>>>(m->P, (const bf16 *)x, dy, n, m->part);
-  k_mlp_reduce<<<(MLP_NPARAM + 255) / 256, 256, 0, s>>>(m->part, ctas, m->grad);
+  k_mlp_reduce<<<(MLP_NPARAM + 31) / 32, 32 * RED_WARPS, 0, s>>>(m->part, ctas, m->grad);
   return cudaGetLastError() == cudaSuccess ? FARGO_OK : FARGO_ERR_CUDA;
 }
 
