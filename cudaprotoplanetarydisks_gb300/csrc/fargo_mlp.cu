@@ -142,15 +142,24 @@ struct MlpBwdW {
   bf16 w3[MLP_H][24];  // W3 [64][8], k (= out) zero-padded to 16; rows of 48 bytes
 };
 
+// W [K][64] (FP32, in-major) into WT [64][K + 8] (BF16, out-major): a thread takes inputs 2m, 2m + 1 of one output; a
+// warp's 8 outputs x 4 pairs fall in 32 different banks (the rows are 4 banks apart mod 32) and
+// read whole 32-byte sectors.  (Element by element, 8-way bank conflicts and a load's latency
+// per element made this prologue most of a small call: 5000 rows 10.4 -> 8.4 us.)
+template <int K, int LD>
+__device__ __forceinline__ void load_transposed(bf16 (*wt)[LD], const float *__restrict__ W, int tid, int nt) {
+  static_assert(LD % 64 == 8, "conflict-free rows");
+#pragma unroll 8
+  for (int e = tid; e < K / 2 * MLP_H; e += nt) {
+    const int t = e & 31, block = e >> 5;  // 8 outputs x 4 pairs
+    const int n = (block & 7) * 8 + (t >> 2), k = 2 * ((block >> 3) * 4 + (t & 3));
+    st_u32(&wt[n][k], pack2(W[k * MLP_H + n], W[(k + 1) * MLP_H + n]));
+  }
+}
+
 __device__ void load_fwd_weights(MlpFwdW &s, const float *__restrict__ P, int tid, int nt) {
-  for (int e = tid; e < MLP_IN * MLP_H; e += nt) {
-    const int k = e / MLP_H, n = e % MLP_H;
-    s.w1t[n][k] = __float2bfloat16_rn(P[MLP_OFF_W1 + e]);
-  }
-  for (int e = tid; e < MLP_H * MLP_H; e += nt) {
-    const int k = e / MLP_H, n = e % MLP_H;
-    s.w2t[n][k] = __float2bfloat16_rn(P[MLP_OFF_W2 + e]);
-  }
+  load_transposed<MLP_IN, MLP_LDX>(s.w1t, P + MLP_OFF_W1, tid, nt);
+  load_transposed<MLP_H, MLP_LDH>(s.w2t, P + MLP_OFF_W2, tid, nt);
   for (int e = tid; e < MLP_H * MLP_OUTP; e += nt) {
     const int k = e / MLP_OUTP, n = e % MLP_OUTP;
     s.w3t[n][k] = __float2bfloat16_rn(n < MLP_OUT ? P[MLP_OFF_W3 + e] : 0.0f);
@@ -163,9 +172,11 @@ __device__ void load_fwd_weights(MlpFwdW &s, const float *__restrict__ P, int ti
 }
 
 __device__ void load_bwd_weights(MlpBwdW &s, const float *__restrict__ P, int tid, int nt) {
-  for (int e = tid; e < MLP_H * MLP_H; e += nt) {
-    const int k = e / MLP_H, n = e % MLP_H;
-    s.w2[k][n] = __float2bfloat16_rn(P[MLP_OFF_W2 + e]);
+#pragma unroll 8
+  for (int e = tid; e < MLP_H * MLP_H / 2; e += nt) {
+    const int k = e / (MLP_H / 2), n = 2 * (e % (MLP_H / 2));
+    const float2 w = *reinterpret_cast<const float2 *>(P + MLP_OFF_W2 + k * MLP_H + n);
+    st_u32(&s.w2[k][n], pack2(w.x, w.y));
   }
   for (int e = tid; e < MLP_H * 24; e += nt) {
     const int k = e / 24, n = e % 24;
