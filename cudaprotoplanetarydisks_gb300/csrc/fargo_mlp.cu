@@ -284,18 +284,21 @@ __device__ __forceinline__ void layers12(const MlpFwdW &s, const bf16 *xs, int l
   }
 }
 
+// Eight warps share a copy of the weights: two CTAs (16 warps) fit an SM, where CTAs of four
+// warps fit three times.  196608 rows 30.7 -> 28.9 us.
+#define FWD_WARPS 8
 struct MlpFwdSmem {
   MlpFwdW w;
-  bf16 xb[4][2][16][MLP_LDX];  // per warp: a double-buffered 16-row tile of X
+  bf16 xb[FWD_WARPS][2][16][MLP_LDX];  // per warp: a double-buffered 16-row tile of X
 };
 
-__global__ void __launch_bounds__(128) k_mlp_forward(const float *__restrict__ P, const bf16 *__restrict__ X, int n,
+__global__ void __launch_bounds__(32 * FWD_WARPS, 2) k_mlp_forward(const float *__restrict__ P, const bf16 *__restrict__ X, int n,
                                                      float *__restrict__ y) {
   extern __shared__ __align__(16) unsigned char mlp_raw[];
   MlpFwdSmem &s = *reinterpret_cast<MlpFwdSmem *>(mlp_raw);
   const int w = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-  const int ntile = (n + 15) / 16, stride = gridDim.x * 4;
-  int tile = blockIdx.x * 4 + w;
+  const int ntile = (n + 15) / 16, stride = gridDim.x * FWD_WARPS;
+  int tile = w * gridDim.x + blockIdx.x;  // few tiles spread over the CTAs
   if (tile < ntile) stage_rows16(&s.xb[w][0][0][0], X, tile * 16, n, lane);
   cp_async_commit();
   load_fwd_weights(s.w, P, threadIdx.x, blockDim.x);
@@ -771,7 +774,7 @@ int fargo_mlp_create(int max_rows, fargo_mlp **out) {
     e = cudaFuncSetAttribute(k_mlp_forward, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fwd_smem());
   if (e == cudaSuccess)
     e = cudaFuncSetAttribute(k_mlp_backward, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bwd_smem());
-  if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_fwd, k_mlp_forward, 128, fwd_smem());
+  if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_fwd, k_mlp_forward, 32 * FWD_WARPS, fwd_smem());
   if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_bwd, k_mlp_backward, 128, bwd_smem());
   if (e == cudaSuccess && (per_fwd < 1 || per_bwd < 1)) e = cudaErrorInvalidConfiguration;
   m->fwd_ctas = sms * per_fwd;
@@ -848,8 +851,8 @@ int fargo_mlp_forward(fargo_mlp *m, const void *x, int n, float *y, int train, v
     const int ctas = std::min(m->tc_ctas, (n + TCF_ROWS - 1) / TCF_ROWS);
     k_mlp_forward_tc<<<ctas, TCF_THREADS, TCF_SMEM, (cudaStream_t)stream>>>(m->P, (const bf16 *)x, n, y, m->err);
   } else {
-    const int warps = (n + 15) / 16, ctas = std::min(m->fwd_ctas, (warps + 3) / 4);
-    k_mlp_forward<<<ctas, 128, fwd_smem(), (cudaStream_t)stream>>>(m->P, (const bf16 *)x, n, y);
+    const int warps = (n + 15) / 16, ctas = std::min(m->fwd_ctas, (warps + 1) / 2);
+    k_mlp_forward<<<ctas, 32 * FWD_WARPS, fwd_smem(), (cudaStream_t)stream>>>(m->P, (const bf16 *)x, n, y);
   }
   return cudaGetLastError() == cudaSuccess ? FARGO_OK : FARGO_ERR_CUDA;
 }
