@@ -49,6 +49,7 @@ enum RingTab {
   RT_AV_R, RT_AV_T,      // 2 CVNR^2 invdiffRmed, 2 CVNR^2/DXTHETA
   RT_AVE_R, RT_AVE_T,    // CVNR^2 invdiffRsup, CVNR^2/DXTHETA
   RT_COOL_S, RT_COOL_I,  // EnergyMed/CoolingTime - QplusMed, 1/CoolingTime (0: no cooling time)
+  RT_SGW, RT_SGW_M,      // weights of the accelerations of rings i and i - 1 at Rinf(i)
   RT_COUNT
 };
 

@@ -403,6 +403,8 @@ void host_ring_table(const fargo_params &p, const HostState &h, const DevParams 
       T(RT_AV_T, i) = 2.0 * FARGO_CVNR * FARGO_CVNR * idx;
       T(RT_AVE_R, i) = FARGO_CVNR * FARGO_CVNR * ids;
       T(RT_AVE_T, i) = FARGO_CVNR * FARGO_CVNR * idx;
+      T(RT_SGW, i) = i > 0 ? (ri - h.Rmed[i - 1]) * idr : 0.0;
+      T(RT_SGW_M, i) = (h.Rmed[i] - ri) * idr;
       T(RT_COOL_S, i) = ct > 0.0 ? T(RT_ENERGYMED, i) / ct - T(RT_QPLUSMED, i) : 0.0;
       T(RT_COOL_I, i) = ct > 0.0 ? 1.0 / ct : 0.0;
     }
