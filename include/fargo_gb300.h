@@ -174,13 +174,13 @@ typedef struct {
   int pad;         /* two substeps per loop iteration, the second with dt = 0 after the DT's last */
   int sg_ahead;    /* the next substep's self-gravity ring transforms beside the end of this one */
   int rotate;      /* rotated DT loop (self-gravity of each substep launched by the previous one) */
-  int az_generic;  /* barrier-per-phase azimuthal transport instead of the register-blocked one */
+  int az_generic;  /* barrier-per-phase azimuthal transport instead of the warp and register-blocked ones */
   int priority;    /* 0 equal stream priorities; 1 hydro chain above self-gravity; 2 the reverse */
   /* tile and launch shapes (each cell's arithmetic unchanged) */
   int cell_block;  /* CTA of the per-cell kernels: 0 64x4 sectors x rings, 1 32x8, 2 128x2, 3 256x1 */
-  int rad_tma;     /* 1: radial transport on TMA-staged tiles in a persistent grid (when the rows
-                      are 16-byte strided); 0: per-thread loads, one CTA per tile */
-  int az_chunks;   /* four-cell chunks per thread of the register azimuthal sweep: 1 (one per
+  int rad_tma;     /* 1: radial transport on TMA-staged tiles in a persistent grid (FP32) or row stages
+                      (FP64), when the rows are 16-byte strided; 0: per-thread loads */
+  int az_chunks;   /* FP32: four-cell chunks per thread of the register azimuthal sweep: 1 (one per
                       thread, up to the CTA size) or 2 (half the threads, two chunks each; the
                       ring mean is summed in another order, so results agree to rounding,
                       not bitwise) */
@@ -188,9 +188,8 @@ typedef struct {
                       of rings with its stencil in registers; no shared memory, no barrier):
                       1 on, 0 off (rad_tma decides), -1 (default) on in FP32-bulk on grids
                       of at least 65536 sectors x ring chunks of 32 (off on smaller grids,
-                      where it has too few threads, and in FP64, where it measured slower
-                      than the TMA-staged tiles); FP32 results are bitwise those of the
-                      tiles, FP64 agree to rounding */
+                      where it has too few threads); bitwise the tiles.  In FP64 every form is
+                      a march: 1 takes its plain loads */
 } fargo_variant;
 /* The default variant, with the FARGO_NO_GRAPH, FARGO_NO_PDL, FARGO_NO_PAD,
    FARGO_NO_SG_AHEAD, FARGO_ROTATE, FARGO_AZ_GENERIC and FARGO_PRIO switches
