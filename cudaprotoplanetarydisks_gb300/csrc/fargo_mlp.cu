@@ -693,33 +693,46 @@ __global__ void __launch_bounds__(128, 2) k_mlp_backward(const float *__restrict
 
 // grad[p] = sum over CTAs c of part[c][p], in a fixed order (deterministic).  A block takes 32
 // parameters; its warp w sums the CTAs w, w + RED_WARPS, ... and the warps' sums are added
-// in order.  The sums are float pairs (Knuth's TwoSum, some 48 bits: rounded to FP32 the
-// FP64 sum's value): this GPU converts 0.6 floats to double per clock and SM, and with one thread
-// per parameter and FP64 sums the conversions and 304 dependent loads took 40 us, now 4 us.
+// in order.  The sums are three floats (Knuth's TwoSum twice, some 70 bits relative to the largest
+// partial sum), added up in FP64 at the end: this GPU converts 0.6 floats to double per clock and
+// SM, and with one thread per parameter and FP64 sums the conversions and 304 dependent loads took
+// 40 us, now 4 us.  Where a float sum leaves FP32's range, or a partial is not finite, the
+// parameter is summed again in FP64 (out of line).
 #define RED_WARPS 8
-struct Sum2 {
-  float hi, lo;
-  __device__ __forceinline__ void add(float x, float xl) {
-    const float t = hi + x, b = t - hi;
-    lo += ((hi - (t - b)) + (x - b)) + xl;
-    hi = t;
+struct Sum3 {
+  float hi, mid, lo;
+  __device__ __forceinline__ static float two_sum(float &s, float x) {
+    const float t = s + x, b = t - s, e = (s - (t - b)) + (x - b);
+    s = t;
+    return e;
   }
+  __device__ __forceinline__ void add(float x) { lo += two_sum(mid, two_sum(hi, x)); }
 };
+__device__ __noinline__ double reduce_any(const float *__restrict__ part, int nparts, int p) {
+  double acc = 0.0;
+  for (int c = 0; c < nparts; c++) acc += (double)part[(size_t)c * MLP_NPARAM + p];
+  return acc;
+}
 __global__ void __launch_bounds__(32 * RED_WARPS) k_mlp_reduce(const float *__restrict__ part, int nparts,
                                                                float *__restrict__ grad) {
-  __shared__ Sum2 sh[RED_WARPS][32];
+  __shared__ Sum3 sh[RED_WARPS][32];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, p = blockIdx.x * 32 + lane;
-  Sum2 s = {0.0f, 0.0f};
+  Sum3 s = {0.0f, 0.0f, 0.0f};
   if (p < MLP_NPARAM) {
 #pragma unroll 8
-    for (int c = w; c < nparts; c += RED_WARPS) s.add(part[(size_t)c * MLP_NPARAM + p], 0.0f);
+    for (int c = w; c < nparts; c += RED_WARPS) s.add(part[(size_t)c * MLP_NPARAM + p]);
   }
   sh[w][lane] = s;
   __syncthreads();
   if (w != 0 || p >= MLP_NPARAM) return;
 #pragma unroll
-  for (int k = 1; k < RED_WARPS; k++) s.add(sh[k][lane].hi, sh[k][lane].lo);
-  grad[p] = s.hi + s.lo;
+  for (int k = 1; k < RED_WARPS; k++) {
+    s.add(sh[k][lane].hi);
+    s.add(sh[k][lane].mid);
+    s.add(sh[k][lane].lo);
+  }
+  const double sum = (double)s.hi + ((double)s.mid + (double)s.lo);
+  grad[p] = (float)(isfinite(s.hi + s.mid + s.lo) ? sum : reduce_any(part, nparts, p));
 }
 
 // Adam (Kingma & Ba 2015) on the FP32 master weights; the padded columns of the
