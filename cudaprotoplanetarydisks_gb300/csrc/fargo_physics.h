@@ -75,8 +75,9 @@ struct Ctl {
   // planetary system (Types.cuh:2-12)
   int nb;
   // 1: the running substep is the last that a reader of the fields can see (the DT's last,
-  // a padded one, one with an error): the fields that no later substep reads
-  // (pressure, temperature, Q+, divergence) are written
+  // a padded one, one entered with an error or a density that is not finite): the fields that no later
+  // substep reads (pressure, temperature, Q+, divergence) are written.  (k_end writes them
+  // when a substep without it fails)
   int diag;
   double x[FARGO_MAXPL], y[FARGO_MAXPL], vx[FARGO_MAXPL], vy[FARGO_MAXPL];
   double mass[FARGO_MAXPL], acc[FARGO_MAXPL];
