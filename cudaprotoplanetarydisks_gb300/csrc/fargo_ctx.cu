@@ -746,6 +746,7 @@ int time_kernels_typed(fargo_ctx *c, int reps, std::vector<double> &ms) {
   int rc = FARGO_OK;
   for (int r = 0; r < reps && rc == FARGO_OK; r++) {
     launch_dt_prefix<T>(a, c->stream);  // a fresh DT per repetition keeps dtemp < DT
+    if (r == reps - 1) CK(cudaMemsetAsync(&c->d_ctl->want_diag, 1, sizeof(int), c->stream));  // fields that a reader sees
     CK(cudaEventRecord(start, c->stream));
     probe.n = 0;
     probe.count = 0;
@@ -1312,6 +1313,7 @@ struct fargo_fused {
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t exec = nullptr;
   std::vector<void *> bufs;  // device: arguments, control-block table, group tables
+  std::vector<Ctl *> ctls;   // the disks' control blocks (on the device)
   int per_substep = 0, per_dt = 0;
   // the launches of the plan, for fused_time_kernels: the DT start, then the
   // substep groups (lane by lane)
@@ -1378,9 +1380,9 @@ int fused_build(fargo_fused *f, fargo_ctx *const *disks, int n, int by_width, st
     return p;
   };
   const KArgs<T> *args_dev = (const KArgs<T> *)dev(args.data(), n * sizeof(KArgs<T>));
-  std::vector<Ctl *> ctls(n);
-  for (int k = 0; k < n; k++) ctls[k] = disks[k]->d_ctl;
-  Ctl *const *ctls_dev = (Ctl *const *)dev(ctls.data(), n * sizeof(Ctl *));
+  f->ctls.resize(n);
+  for (int k = 0; k < n; k++) f->ctls[k] = disks[k]->d_ctl;
+  Ctl *const *ctls_dev = (Ctl *const *)dev(f->ctls.data(), n * sizeof(Ctl *));
   if (!args_dev || !ctls_dev) {
     *why = "device allocation of the fused plan failed";
     return FARGO_ERR_CUDA;
@@ -1648,6 +1650,8 @@ int fused_time_kernels(fargo_fused *f, int reps, double *ms, int cap, int *ngrou
   std::vector<double> acc(G, 0.0);
   int rc = FARGO_OK;
   for (int r = 0; r < reps && rc == FARGO_OK; r++) {
+    for (Ctl *c : f->ctls)
+      if (r == reps - 1) cudaMemsetAsync(&c->want_diag, 1, sizeof(int), f->stream);  // fields that a reader sees
     cudaEventRecord(ev[0], f->stream);
     for (int q = 0; q < G; q++) {
       f->body[q].fn(f->stream, 0);

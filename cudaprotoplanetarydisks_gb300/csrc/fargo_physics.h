@@ -87,7 +87,7 @@ struct Ctl {
   // per-substep planet parameters, computed once after each planet update:
   // bodies feeling the disk (0 = the star) and the potential of every planet
   int nbody;
-  int pad2;
+  int want_diag;              // 1: diag whatever the substep is (the last one of a timed run); until the next DT begins
   double bx[FARGO_MAXPL + 1], by[FARGO_MAXPL + 1], brs2[FARGO_MAXPL + 1];
   double px[FARGO_MAXPL], py[FARGO_MAXPL], pm[FARGO_MAXPL], ps2[FARGO_MAXPL], pinvd3[FARGO_MAXPL];
   // disk accelerations of the bodies (ComputeAccel) and start time of the substep
