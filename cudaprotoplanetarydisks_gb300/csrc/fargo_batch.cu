@@ -49,7 +49,7 @@ int fargo_batch_create_variant(int n, const fargo_params *params, const fargo_pl
     fargo_ctx *c = nullptr;
     const long long others = cells - (long long)params[k].nrad * params[k].nsec;
     const int rc = fargo_ctx_create_among(&params[k], nplanets[k] ? planets + off : nullptr, nplanets[k], precision,
-                                          nullptr, v, others, &c);
+                                          nullptr, v, others, 0, &c);
     if (rc != FARGO_OK) {
       fargo_batch_destroy(b);
       return rc;

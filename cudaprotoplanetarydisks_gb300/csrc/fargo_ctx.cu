@@ -84,7 +84,7 @@ struct fargo_ctx {
   int az_chunks = 1;          // chunks per thread of the register azimuthal sweep
   long long others = 0;       // cells of the disks that run at the same time (an ensemble)
   bool gas = false;           // FP32, large grids: source step to energy equation by k_gas
-  int gas_rings = 4;          // its rings per chunk
+  int gas_rings = 0;          // its rings per chunk
   int rad_rings = 4;          // FP64: rings per chunk of the radial march
   bool rad_col = false;       // column-march radial transport
 };
@@ -509,12 +509,13 @@ int init_typed(fargo_ctx *c, const fargo_planet *planets) {
     // k_gas where the disks that run at the same time have a million cells: below, its
     // blocks are too few to hide a march's latency (one disk of 512 x 1536: a substep 98 us
     // with the cell kernels, 109 with k_gas; 640 x 1920: 58 against 49 ms for five DTs; 1024 x 3072: 380
-    // against 344 us; 32 disks of 128 to 512 rings: 207 against 172 ms for five DTs).  In an ensemble the
-    // disks fill the GPU together and chunks of 16 rings measured best (8 .. 64).
-    c->gas = E == 4 && (long long)p.nrad * p.nsec + c->others >= GAS_CELLS;
+    // against 344 us; 32 disks of 128 to 512 rings: 207 against 172 ms for five DTs).  In an ensemble
+    // smaller disks fill the GPU together and chunks of 16 rings measured best (8 .. 64); a disk of a
+    // million cells keeps the chunks it takes alone, which fill the GPU by itself.
+    c->gas = E == 4 && (c->gas_rings || (long long)p.nrad * p.nsec + c->others >= GAS_CELLS);
     for (int k = 0; k < 2 && c->gas && c->az_warp32; k++)
       if ((rc = dev_alloc(c, &c->mom_extra[k], sg * E))) return rc;
-    c->gas_rings = c->others ? 16 : gas_rings(p.nrad, p.nsec, sms);
+    if (!c->gas_rings) c->gas_rings = (long long)p.nrad * p.nsec < GAS_CELLS ? 16 : gas_rings(p.nrad, p.nsec, sms);
   }
   // TMA maps of the radial transport's input fields
   if (c->want_tma) make_rad_maps<T>(c);
@@ -830,11 +831,11 @@ int fargo_ctx_create(const fargo_params *p, const fargo_planet *planets, int nb,
 
 int fargo_ctx_create_variant(const fargo_params *p, const fargo_planet *planets, int nb, int precision, void *stream,
                              const fargo_variant *variant, fargo_ctx **out) {
-  return fargo_ctx_create_among(p, planets, nb, precision, stream, variant, 0, out);
+  return fargo_ctx_create_among(p, planets, nb, precision, stream, variant, 0, 0, out);
 }
 
 int fargo_ctx_create_among(const fargo_params *p, const fargo_planet *planets, int nb, int precision, void *stream,
-                           const fargo_variant *variant, long long others, fargo_ctx **out) {
+                           const fargo_variant *variant, long long others, int gas_rings, fargo_ctx **out) {
   if (!p || !out || nb < 0 || nb > FARGO_MAXPL || (nb > 0 && !planets)) return FARGO_ERR_INVALID;
   fargo_variant v;
   if (variant) v = *variant;
@@ -850,6 +851,7 @@ int fargo_ctx_create_among(const fargo_params *p, const fargo_planet *planets, i
   c->precision = precision;
   c->esize = precision == FARGO_FP64 ? 8 : 4;
   c->others = others;
+  c->gas_rings = gas_rings < 0 ? 0 : gas_rings > GAS_MAX_RINGS ? GAS_MAX_RINGS : gas_rings;
   c->dp = host_dev_params(*p, nb);
   c->use_graph = v.graph != 0;
   c->use_pdl = v.pdl != 0;

@@ -93,9 +93,11 @@ struct DiskView {
   double *ring;
   void *cand;
 };
-// fargo_ctx_create_variant for a disk that runs beside others of that many cells together
+// fargo_ctx_create_variant for a disk that runs beside others of that many cells together.  gas_rings > 0: an FP32
+// disk of any size takes k_gas, with chunks of that many rings (for tests); 0: by the disks' sizes
 extern "C" int fargo_ctx_create_among(const fargo_params *p, const fargo_planet *planets, int nb, int precision, void *stream,
-                                      const fargo_variant *variant, long long others, fargo_ctx **out);
+                                      const fargo_variant *variant, long long others, int gas_rings,
+                                      fargo_ctx **out);
 extern "C" int fargo_disk_view(fargo_ctx *c, DiskView *v);
 
 // output.cpp
