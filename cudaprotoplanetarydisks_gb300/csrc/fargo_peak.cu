@@ -1,5 +1,6 @@
 // Measured FP64-pipe peak of the current device (fargo_fp64_pipe_peak), and the
-// self-test of the step's FP64 divides (fargo_div_selftest).
+// self-tests of the step's FP64 divides (fargo_div_selftest) and of its arithmetic in float
+// pairs (fargo_pair_selftest).
 //
 // GB300 issues FP64 arithmetic on a narrow pipe (about two lanes per clock per
 // SM), and the FP64 mode of the hydro step is bound by it, not by HBM.  Its
@@ -86,6 +87,83 @@ extern "C" int fargo_div_selftest(const double *a, const double *b, int n, doubl
     if (cudaDeviceSynchronize() != cudaSuccess ||
         cudaMemcpy(q_step, d + 2 * (size_t)n, bytes, cudaMemcpyDeviceToHost) != cudaSuccess ||
         cudaMemcpy(q_lim, d + 3 * (size_t)n, bytes, cudaMemcpyDeviceToHost) != cudaSuccess)
+      rc = FARGO_ERR_CUDA;
+  }
+  cudaFree(d);
+  return rc;
+}
+
+namespace {
+// in: 4 doubles per case
+__global__ void k_pair_selftest(int which, const double *__restrict__ in, int n, double *__restrict__ out) {
+  const int k = blockIdx.x * blockDim.x + threadIdx.x;
+  if (k >= n) return;
+  const double a = in[4 * k], b = in[4 * k + 1], c = in[4 * k + 2], d = in[4 * k + 3];
+  float ch, cl, rh, rl;
+  limiter_coefficient(fabs(c), c < 0.0 ? 0x80000000u : 0u, ch, cl);
+  double y = 0.0;
+  switch (which) {
+    case FARGO_PAIR_RCP: y = frcp64(a); break;
+    case FARGO_PAIR_RSQRT: y = rsqrt64(a); break;
+    case FARGO_PAIR_JOIN: y = join_scaled((float)a, (float)b, 0u); break;
+    case FARGO_PAIR_LIMITER: y = limiter_fraction(a, b, ch, cl); break;
+    case FARGO_PAIR_LIMITER_SCALED:
+      split_pair(d, rh, rl);
+      y = limiter_fraction_scaled(a, b, rh, rl, d, ch, cl);
+      break;
+    case FARGO_PAIR_DIFF: {
+      Split3 p, q;
+      const bool in_range = split3(a, p) & split3(b, q);
+      const float2 x = diff_pair(p, q);
+      y = in_range ? (double)x.x + (double)x.y : __longlong_as_double(0x7ff8000000000000LL);
+      break;
+    }
+    case FARGO_PAIR_STAR: {
+      Split3 p, q, r;
+      split3(a, p);
+      split3(b, q);
+      split3(d, r);
+      y = star_pair(b, diff_pair(r, q), diff_pair(q, p), ch, cl);
+      break;
+    }
+    case FARGO_PAIR_FP32_QUOTIENT: {
+      f32::Noted noted;
+      y = (double)noted.div((float)a, (float)b);
+      break;
+    }
+    case FARGO_PAIR_FP32_MISMATCHES: {
+      // 4096 random pairs of significands, the divisor's exponent in -60 .. 120 and the quotient's in -40 .. 40
+      unsigned long long x = (unsigned long long)a + 0x9e3779b97f4a7c15ull * (k + 1);
+      f32::Noted noted;
+      int bad = 0;
+      for (int i = 0; i < 4096; i++) {
+        x ^= x << 13;
+        x ^= x >> 7;
+        x ^= x << 17;
+        const int e = (int)((x >> 46) % 181) - 60, f = (int)((x >> 54) % 81) - 40 + e;
+        const float v = __uint_as_float(((unsigned)(127 + e) << 23) | (unsigned)(x & 0x7fffff));
+        const int g = f < -102 ? -102 : f > 126 ? 126 : f;
+        const float u = __uint_as_float(((unsigned)(127 + g) << 23) | (unsigned)(x >> 23 & 0x7fffff));
+        if (noted.div(u, v) != __fdiv_rn(u, v)) bad++;
+      }
+      y = bad;
+      break;
+    }
+  }
+  out[k] = y;
+}
+}  // namespace
+
+extern "C" int fargo_pair_selftest(int which, const double *in, int n, double *out) {
+  if (!in || !out || n < 1 || n > (1 << 22) || which < 0 || which > FARGO_PAIR_FP32_MISMATCHES) return FARGO_ERR_INVALID;
+  double *d = nullptr;
+  const size_t bytes = (size_t)n * sizeof(double);
+  if (cudaMalloc(&d, 5 * bytes) != cudaSuccess) return FARGO_ERR_CUDA;
+  int rc = cudaMemcpy(d, in, 4 * bytes, cudaMemcpyHostToDevice) == cudaSuccess ? FARGO_OK : FARGO_ERR_CUDA;
+  if (rc == FARGO_OK) {
+    k_pair_selftest<<<(n + 127) / 128, 128>>>(which, d, n, d + 4 * (size_t)n);
+    if (cudaDeviceSynchronize() != cudaSuccess ||
+        cudaMemcpy(out, d + 4 * (size_t)n, bytes, cudaMemcpyDeviceToHost) != cudaSuccess)
       rc = FARGO_ERR_CUDA;
   }
   cudaFree(d);

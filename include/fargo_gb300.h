@@ -298,12 +298,24 @@ const char *fargo_substep_kernel_name(const fargo_ctx *ctx, int k);
    of the FP64 mode, whose kernels are bound by this pipe.  Synchronous. */
 int  fargo_fp64_pipe_peak(double *dfma_per_s);
 /* Self-test of the FP64 step's two divides on the device: q_step[k] = a[k] / b[k]
-   as the per-cell arithmetic divides (the reciprocal estimate, one Newton step,
-   the quotient and one correction: the correctly rounded quotient except within
-   about 2^-80 of a rounding midpoint) and q_lim[k] as the slope limiters divide
-   (without the correction: relative error about 2^-40); both IEEE a / b outside
-   |a|, |b| in [2^-500, 2^501).  n in 1..2^24.  Synchronous. */
+   as the per-cell arithmetic divides (a reciprocal within 2^-44 formed in a pair of floats, the
+   quotient and one correction: the correctly rounded quotient except within
+   about 2^-88 of a rounding midpoint) and q_lim[k] as the slope limiters of the
+   barrier-per-phase azimuthal kernel divide (without the correction: relative error about
+   2^-44); both IEEE a / b outside |a|, |b| in [2^-500, 2^501).  n in 1..2^24.  Synchronous. */
 int  fargo_div_selftest(const double *a, const double *b, int n, double *q_step, double *q_lim);
+/* Self-test of the steps' arithmetic in float pairs on the device: out[k] from the four doubles
+   (a, b, c, d) at in[4 k], |c| <= 2.  n in 1..2^22.  Synchronous. */
+#define FARGO_PAIR_RCP             0  /* 1 / a */
+#define FARGO_PAIR_RSQRT           1  /* 1 / sqrt(a) */
+#define FARGO_PAIR_JOIN            2  /* the double of the floats a + b */
+#define FARGO_PAIR_LIMITER         3  /* c b / (a + b), a and b of one sign */
+#define FARGO_PAIR_LIMITER_SCALED  4  /* c d b / (a + d b) */
+#define FARGO_PAIR_DIFF            5  /* a - b; NaN where the pairs do not take a or b */
+#define FARGO_PAIR_STAR            6  /* b + c x y / (x + y), x = d - b and y = b - a of one sign; else b */
+#define FARGO_PAIR_FP32_QUOTIENT   7  /* the FP32 march's a / b */
+#define FARGO_PAIR_FP32_MISMATCHES 8  /* of 4096 random FP32 pairs (seed a), those whose quotient is not IEEE's */
+int  fargo_pair_selftest(int which, const double *in, int n, double *out);
 /* Self-test of the 5th-generation tensor-core path (tcgen05, sm_100 family): one
    CTA computes d (128 x n, FP32, row-major) = a (128 x k, BF16 bit patterns,
    row-major) x b (n x k, BF16, row-major)^T with k / 16 MMAs accumulating in
