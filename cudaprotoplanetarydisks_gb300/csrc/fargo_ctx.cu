@@ -1357,7 +1357,7 @@ int fused_build(fargo_fused *f, fargo_ctx *const *disks, int n, int by_width, st
     const char *no = p.self_gravity ? "self-gravity"
                    : (p.open_inner || p.non_reflecting || p.evanescent) ? "an open, non-reflecting or evanescent boundary"
                    : p.sloppy_cfl ? "the sloppy CFL (-c)"
-                   : !c->az_regs ? "a ring too wide for the register azimuthal sweep"
+                   : !c->az_regs ? "a ring that is no multiple of four sectors, too wide, or swept by the barrier-per-phase kernel"
                    : nullptr;
     if (no) {
       *why = "disk " + std::to_string(k) + " uses " + no + ", which the fused form does not carry";
@@ -1441,7 +1441,7 @@ int fused_build(fargo_fused *f, fargo_ctx *const *disks, int n, int by_width, st
     return make_int2(gas_columns_host(p.nsec), (p.nrad + c->gas_rings - 1) / c->gas_rings);
   };
   auto corot = [](const fargo_params &p, const fargo_ctx *) { return p.corotating != 0; };
-  auto az_mc = [](const fargo_params &p, const fargo_ctx *) { return sizeof(T) == 4 && p.nsec / 4 > az4_threads_host<T>(p.nsec); };
+  auto az_mc = [](const fargo_params &p, const fargo_ctx *) { return sizeof(T) == 4 && p.nsec / 4 > az4_threads(p.nsec); };
   auto az_one = [&](const fargo_params &p, const fargo_ctx *c) { return !az_mc(p, c); };
   auto az_grid = [](const fargo_params &p, const fargo_ctx *) {
     return make_int2(p.nrad, sizeof(T) == 8 ? azw_blocks_host(p.nsec) : 1);
@@ -1458,7 +1458,7 @@ int fused_build(fargo_fused *f, fargo_ctx *const *disks, int n, int by_width, st
       const fargo_params &p = disks[k]->P;
       if (w && p.nsec != w) continue;
       if (v4(p, disks[k])) v4_threads = std::max(v4_threads, (p.nsec / 4 + 31) / 32 * 32);
-      az_threads = std::max(az_threads, sizeof(T) == 8 ? azw_threads_host(p.nsec) : az4_threads_host<T>(p.nsec));
+      az_threads = std::max(az_threads, sizeof(T) == 8 ? azw_threads_host(p.nsec) : az4_threads(p.nsec));
       az_smem = std::max(az_smem, disks[k]->az_smem);
     }
     body.push_back({group(BK_CFL_V4, w, v4, rings, dim3(v4_threads), 0, 0),

@@ -156,8 +156,7 @@ void launch_batched(int kernel, const BatchGroup<T> &G, int nblocks, dim3 block,
 void launch_loop_cond(Ctl *const *ctls, int n, unsigned long long handle, int pdl, cudaStream_t s);
 template <class T>
 cudaError_t prepare_batched(size_t rad_smem, size_t az_smem);
-template <class T>
-int az4_threads_host(int nsec);
+int az4_threads(int nsec);
 // the warp azimuthal kernel's blocks per ring and threads per block
 int azw_blocks_host(int nsec);
 int azw_threads_host(int nsec);

@@ -372,8 +372,9 @@ int  fargo_batch_create_variant(int n, const fargo_params *params, const fargo_p
    lane (one launch per kernel for the whole ensemble, blocks shaped for the
    widest ring).  Bitwise the results of the disks run alone.
    FARGO_ERR_INVALID (reason in fargo_batch_last_error) when a disk uses
-   self-gravity, an open, non-reflecting or evanescent boundary, the sloppy CFL
-   or a ring too wide for the register azimuthal sweep. */
+   self-gravity, an open, non-reflecting or evanescent boundary, the sloppy CFL, the
+   barrier-per-phase azimuthal sweep, or a ring that is no multiple of four sectors or too
+   wide (13 of its rows have to fit in shared memory). */
 int  fargo_batch_fuse(fargo_batch *b);
 int  fargo_batch_fuse_by_width(fargo_batch *b, int by_width);
 /* The reason of the last failed fargo_batch_fuse ("" if none). */
