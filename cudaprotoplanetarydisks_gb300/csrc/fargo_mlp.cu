@@ -696,7 +696,7 @@ __global__ void __launch_bounds__(128, 2) k_mlp_backward(const float *__restrict
 // in order.  The sums are three floats (Knuth's TwoSum twice, some 70 bits relative to the largest
 // partial sum), added up in FP64 at the end: this GPU converts 0.6 floats to double per clock and
 // SM, and with one thread per parameter and FP64 sums the conversions and 304 dependent loads took
-// 40 us, now 4 us.  Where a float sum leaves FP32's range, or a partial is not finite, the
+// 40 us, now 11 with a cold cache.  Where a float sum leaves FP32's range, or a partial is not finite, the
 // parameter is summed again in FP64 (out of line).
 #define RED_WARPS 8
 struct Sum3 {
